@@ -950,8 +950,10 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
                 fold();
                 flush_warp<MODEL>(sh.fit[group], cur_chunks, sh.pub[group][0]);
                 cur_chunks = 0;
-                group_sync();
             }
+            // For every warp of the group, also one that the former fit's tiles
+            // had no chunk for: fit[] and pub[] are written anew below.
+            if (cur_fit >= 0) group_sync();
             if (gw == 0) {
                 const FitDev& fg = fits[tile.fit];
                 if (lane < (int)(sizeof(FitDev) / 8))
