@@ -596,6 +596,11 @@ struct mc_model {
         if (tiles_ready && plan.narrow_window <= batch.narrow_window && plan.narrow_sessions >= batch.narrow_sessions) return MC_OK;
         return build_tiles(layout_model, batch.narrow_sessions);
     }
+    // A shape that was refused leaves a tile fit without tiles.
+    int need_tiles(const char* who) const {
+        if (d_coff || tiles_ready) return MC_OK;
+        return set_error(MC_ERR_STATE, std::string(who) + ": no tiles (the last tile shape was refused; configure another)");
+    }
     FitDev make_desc() const;
     int write_fit_desc();
     // Every parameter at its prior value 1/2 (the default Param (1, 2), param.cuh:18-39)
@@ -1418,6 +1423,7 @@ extern "C" int mc_model_em(mc_model* m, int32_t iters, int impl, void* stream) {
         // The count path (PBM/UBM) does not depend on the session order.
         if (!m->fused_ok && !m->d_coff)
             return set_error(MC_ERR_INVALID, "model_em: fused path unavailable: " + m->fused_reason);
+        if (int rc = m->need_tiles("model_em")) return rc;
         // The loop is captured as graphs of at most kGraphChunk iterations
         // (one full chunk, one remainder), each replayed as often as needed.
         const int full = iters / kGraphChunk, rem = iters % kGraphChunk;
@@ -1654,6 +1660,7 @@ extern "C" int mc_model_em_trace(mc_model* m, int32_t iters, double* train_ll, v
         for (int i = 0; i < iters; i++) train_ll[i] = 0.0;
         return MC_OK;
     }
+    if (int rc = m->need_tiles("em_trace")) return rc;
     double* d_trace = nullptr;
     int64_t scratch = 0;
     int rc = dalloc(&d_trace, (size_t)iters * (MC_R + 1), &scratch);

@@ -66,3 +66,18 @@ def test_more_wide_tiles_than_ctas_over_many_fits(models):
     for k, (f, cm) in enumerate(zip(fits, batch_models)):
         _check(cm, *f, 4, f"fit {k}")
     batch.close()
+
+
+def test_em_after_a_refused_shape_is_an_error():
+    """A window that no CTA holds: configure refuses it, and EM has no tiles to
+    run over until another shape is set."""
+    sessions, n_qd = _sessions([(40, 90, 0.8), (12, 30, 0.5)], 1)
+    cm = _upload(api.DBN, sessions, n_qd)
+    with pytest.raises(api._capi.MCError):
+        cm.configure(0, 16384, 0)
+    for call in (lambda: cm.em(1), lambda: cm.em_trace(1)):
+        with pytest.raises(api._capi.MCError):
+            call()
+    cm.configure(0, WINDOW, 0)
+    cm.em(3)
+    _check(cm, api.DBN, sessions, n_qd, 3, "after a refused shape")
