@@ -269,8 +269,9 @@ typedef struct mc_batch mc_batch;
  * (mc_model_fused_path = 0) share one persistent tile launch and are given the
  * first such model's tile shape; models on the count path (PBM, UBM) share
  * one batched count launch.  Models keep their own parameters and may still
- * be used alone; they must not be re-uploaded or reconfigured while the batch
- * exists. */
+ * be used alone, or be in several batches, advanced in turn; they must not be
+ * re-uploaded or reconfigured while a batch with them exists.  A batch cuts
+ * tiles of its own for models whose tiles its launches would not take well. */
 int mc_batch_create(int n_models, mc_model* const* models, mc_batch** out);
 
 /* n_iterations fused iterations of every model, captured as CUDA graphs and

@@ -17,6 +17,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <thread>
 #include <vector>
@@ -409,6 +410,33 @@ static bool fused_plan(int model, int wqd, int spt, int block, int device, bool 
            plan->ctas >= 1 && plan->cap >= widest + 8;
 }
 
+// Tiles cut from a model's blocks for one kind of launch, packed on the device.
+// A model holds its own; a batch holds those that its launches take, so a set
+// outlives a model's change to another while a batch still runs over it.
+struct TileSet {
+    TileDev* d_tiles = nullptr;
+    SplitDev* d_splits = nullptr;
+    double* d_split_bins = nullptr;
+    unsigned* d_split_count = nullptr;
+    unsigned char* d_tblk = nullptr;
+    int n_tiles = 0, n_wide = 0, n_splits = 0, n_echunks = 0;
+    int widest = 0;  // widest staged window of the wide tiles
+    int narrow_window = 0, narrow_sessions = 0;  // the limits it was cut with
+    int64_t bytes = 0;
+
+    TileSet() = default;
+    TileSet(const TileSet&) = delete;
+    TileSet& operator=(const TileSet&) = delete;
+    ~TileSet() {
+        settle(d_tiles, d_splits, d_split_bins, d_split_count, d_tblk);
+        dfree(d_tiles);
+        dfree(d_splits);
+        dfree(d_split_bins);
+        dfree(d_split_count);
+        dfree(d_tblk);
+    }
+};
+
 struct HostState {
     int status, iter, pad[2];
     float theta[2 * MC_MAX_PUB];  // the half (iter & 1) is current
@@ -424,7 +452,7 @@ struct mc_model {
     PinnedArray<int32_t> seg_lo, seg_hi;  // qd range [lo, hi) of each segment, as the upload pass finds it
     PinnedArray<uint32_t> packbits;  // bit s: training session s has a click
     int spt = 1024, wqd = 1536, block = 256;
-    FusedPlan plan;  // of the tiles built
+    FusedPlan plan;  // of the model's own launches over `tiles`
     // fused state
     int32_t* d_pidx = nullptr;
     uint16_t* d_click = nullptr;
@@ -435,20 +463,15 @@ struct mc_model {
     DenseTable dense{};            // PBM: counts by rank (when all fit 16 bits)
     int64_t n_cent = 0;
     float *d_atr = nullptr, *d_sat = nullptr, *d_pub_theta = nullptr;
-    double *d_pub_bins = nullptr, *d_pub_const = nullptr, *d_split_bins = nullptr;
-    unsigned *d_split_count = nullptr, *d_tiles_done = nullptr;
+    double *d_pub_bins = nullptr, *d_pub_const = nullptr;
+    unsigned* d_tiles_done = nullptr;
     // Status word, iterations completed and public values in one block, which
     // one copy reads back (HostState); d_status, d_iter and d_pub_theta lie in it.
     int* d_state = nullptr;
     int *d_iter = nullptr, *d_status = nullptr;
     FitDev* d_fit = nullptr;
-    TileDev* d_tiles = nullptr;
-    SplitDev* d_splits = nullptr;
     WorkState* d_ws = nullptr;
-    int n_tiles = 0, n_wide = 0, n_splits = 0, n_echunks = 0;
-    int widest = 0;        // widest staged window of the wide tiles
-    int tiles_layout = 0;  // kernel (model, or -1) that the tiles were laid out for
-    bool tiles_ready = false;  // tiles built for the current shape (PBM/UBM build them only for batches)
+    std::shared_ptr<TileSet> tiles;  // for the current shape and the model's own launches (count-path models: none)
     // The adjoint's tiles, a block of threads each: the blocks that the EM
     // tiles are cut from, with their first sessions in ascending order (range
     // lookups).  On the first call for an FP32 gradient: the per-tile counts
@@ -466,9 +489,6 @@ struct mc_model {
     // Launch shapes of the count kernels (entry kernel; dense PBM kernel).
     CountShape count_shape{8, 256, 8};
     CountShape dense_shape{0, 256, 6};
-    unsigned char* d_tblk = nullptr;
-    int64_t split_bins_count = 0;
-    int64_t tile_bytes = 0;
     // plain state (allocated on first use)
     PlainRec* d_recs = nullptr;
     float2 *d_atr2 = nullptr, *d_sat2 = nullptr, *d_pub2 = nullptr, *d_tmp_atr = nullptr, *d_tmp_sat = nullptr,
@@ -522,15 +542,8 @@ struct mc_model {
         int n_wide = 0;
     };
     void free_tiles() {
-        settle(d_tiles, d_splits, d_split_bins, d_split_count, d_tblk);
-        dfree(d_tiles);
-        dfree(d_splits);
-        dfree(d_split_bins);
-        dfree(d_split_count);
-        dfree(d_tblk);
-        bytes -= tile_bytes;
-        tile_bytes = 0;
-        tiles_ready = false;
+        if (tiles) bytes -= tiles->bytes;
+        tiles.reset();
         settle(d_adj_off, d_adj_cnt, d_adj_tiles, d_adj_blk);
         dfree(d_adj_off);
         dfree(d_adj_cnt);
@@ -580,28 +593,15 @@ struct mc_model {
 
     int64_t qd_alloc() const { return ((std::max<int64_t>(n_qd, 1) + 3) & ~(int64_t)3) + 4; }
     void cut_tiles(int narrow_window, int narrow_sessions, TileList& out);
-    int build_tiles(int layout_model, int narrow_sessions);  // narrow_sessions 0: the plan's
-    int build_tiles() { return build_tiles(model, 0); }
-    // Tiles for the tile kernel (batched launches, autotuning): built at upload
-    // for DBN/CCM, on first use for the count-path models.
-    int ensure_tiles() {
-        if (!fused_ok) return set_error(MC_ERR_INVALID, "tile path unavailable: " + fused_reason);
-        return tiles_ready ? MC_OK : build_tiles();
-    }
-    // Tiles for a batch's launches: cut again where the batch's narrow tiles
-    // hold less (a model of its own in a mixed batch), or fewer sessions were
-    // taken per tile than the batch as a whole wants.
-    int ensure_tiles(const FusedPlan& batch, int layout_model) {
-        if (!fused_ok) return set_error(MC_ERR_INVALID, "tile path unavailable: " + fused_reason);
-        if (tiles_ready && plan.narrow_window <= batch.narrow_window && plan.narrow_sessions >= batch.narrow_sessions) return MC_OK;
-        return build_tiles(layout_model, batch.narrow_sessions);
-    }
+    int build_tiles();
+    int pack_set(TileList& list, TileSet& set);
+    int batch_tiles(const FusedPlan& batch, std::shared_ptr<TileSet>* out);
     // A shape that was refused leaves a tile fit without tiles.
     int need_tiles(const char* who) const {
-        if (d_coff || tiles_ready) return MC_OK;
+        if (d_coff || tiles) return MC_OK;
         return set_error(MC_ERR_STATE, std::string(who) + ": no tiles (the last tile shape was refused; configure another)");
     }
-    FitDev make_desc() const;
+    FitDev make_desc(const TileSet* set) const;
     int write_fit_desc();
     // Every parameter at its prior value 1/2 (the default Param (1, 2), param.cuh:18-39)
     // and the iteration counter at 0, queued on st.
@@ -854,58 +854,69 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
     });
 }
 
-// The EM kernel's tiles, laid out for the kernel of layout_model (the model's
-// own, or -1, the model-generic one of mixed batches), and the adjoint's, which
-// are their blocks.
-int mc_model::build_tiles(int layout_model, int narrow_sessions) {
-    drop_graph();
-    free_tiles();
-    const std::string misfit = "tile shape does not fit in shared memory (reduce sessions per tile or window)";
-    if (!fused_plan(layout_model, wqd, spt, block, device, false, n, 0, &plan)) return set_error(MC_ERR_INVALID, misfit);
-    TileList list;
-    if (narrow_sessions) plan.narrow_sessions = narrow_sessions;
-    const int narrow = plan.narrow_sessions;
-    cut_tiles(plan.narrow_window, narrow, list);
+// A set's device arrays and packed sessions from its list; the adjoint's tiles
+// (d_adj_tiles), which are the list's blocks, have to be there.
+int mc_model::pack_set(TileList& list, TileSet& set) {
     std::vector<TileDev>& tiles = list.tiles;
-    widest = 0;
-    for (int k = 0; k < list.n_wide; k++)
-        if (tiles[(size_t)k].qd_count <= wqd) widest = std::max(widest, tiles[(size_t)k].qd_count);
-    if (!fused_plan(layout_model, wqd, spt, block, device, false, n, widest, &plan)) return set_error(MC_ERR_INVALID, misfit);
-    plan.narrow_sessions = narrow;
-    const std::vector<SplitDev>& splits = list.splits;
-    const int64_t bin_off = list.split_bins;
     // Packed session blocks of the staged (non-direct) tiles, 16-byte aligned.
     // Sized by the packed counts, which the packing kernel checks.
     int64_t blk = 0;
     int max_tile_sessions = 1;
-    n_echunks = 0;
-    for (TileDev& t : tiles) {
+    for (size_t k = 0; k < tiles.size(); k++) {
+        TileDev& t = tiles[k];
         t.blk_off = blk;
         if (t.qd_count <= wqd) {
             blk += (int64_t)kChunkBytes * ((t.s_packed + 31) / 32);
             max_tile_sessions = std::max(max_tile_sessions, t.s_count);
+            if (k < (size_t)list.n_wide) set.widest = std::max(set.widest, t.qd_count);
         }
         // E-step chunks of 32 sessions, at least one per tile
-        n_echunks += std::max(1, ((t.qd_count <= wqd ? t.s_packed : t.s_count) + 31) / 32);
+        set.n_echunks += std::max(1, ((t.qd_count <= wqd ? t.s_packed : t.s_count) + 31) / 32);
     }
-    n_tiles = (int)tiles.size();
-    n_wide = list.n_wide;
-    n_splits = (int)splits.size();
-    split_bins_count = bin_off;
-    int64_t before = bytes;
+    set.n_tiles = (int)tiles.size();
+    set.n_wide = list.n_wide;
+    set.n_splits = (int)list.splits.size();
     int rc;
-    if ((rc = dalloc(&d_tiles, tiles.size(), &bytes))) return rc;
-    if ((rc = dalloc(&d_splits, splits.size(), &bytes))) return rc;
-    if ((rc = dalloc(&d_split_bins, (size_t)bin_off, &bytes))) return rc;
-    if ((rc = dalloc(&d_split_count, splits.size(), &bytes))) return rc;
-    if ((rc = dalloc(&d_tblk, (size_t)std::max<int64_t>(blk, 16), &bytes))) return rc;
-    tile_bytes = bytes - before;
-    if (!tiles.empty()) CK(cudaMemcpy(d_tiles, tiles.data(), tiles.size() * sizeof(TileDev), cudaMemcpyHostToDevice));
-    if (!splits.empty()) CK(cudaMemcpy(d_splits, splits.data(), splits.size() * sizeof(SplitDev), cudaMemcpyHostToDevice));
-    CK(cudaMemset(d_split_bins, 0, (size_t)std::max<int64_t>(bin_off, 1) * sizeof(double)));
-    CK(cudaMemset(d_split_count, 0, std::max<size_t>(splits.size(), 1) * sizeof(unsigned)));
-    int rc2 = write_fit_desc();
-    if (rc2) return rc2;
+    if ((rc = dalloc(&set.d_tiles, tiles.size(), &set.bytes))) return rc;
+    if ((rc = dalloc(&set.d_splits, list.splits.size(), &set.bytes))) return rc;
+    if ((rc = dalloc(&set.d_split_bins, (size_t)list.split_bins, &set.bytes))) return rc;
+    if ((rc = dalloc(&set.d_split_count, list.splits.size(), &set.bytes))) return rc;
+    if ((rc = dalloc(&set.d_tblk, (size_t)std::max<int64_t>(blk, 16), &set.bytes))) return rc;
+    if (!tiles.empty()) CK(cudaMemcpy(set.d_tiles, tiles.data(), tiles.size() * sizeof(TileDev), cudaMemcpyHostToDevice));
+    if (!list.splits.empty())
+        CK(cudaMemcpy(set.d_splits, list.splits.data(), list.splits.size() * sizeof(SplitDev), cudaMemcpyHostToDevice));
+    CK(cudaMemset(set.d_split_bins, 0, (size_t)std::max<int64_t>(list.split_bins, 1) * sizeof(double)));
+    CK(cudaMemset(set.d_split_count, 0, std::max<size_t>(list.splits.size(), 1) * sizeof(unsigned)));
+    int* d_occ = nullptr;
+    int64_t scratch = 0;
+    if ((rc = dalloc(&d_occ, list.blocks.size(), &scratch))) return rc;
+    cudaError_t e = cudaSuccess;
+    auto ck = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
+    ck(cudaMemsetAsync(d_occ, 0, std::max<size_t>(list.blocks.size(), 1) * sizeof(int), 0));
+    ck(launch_tile_occ(model, d_adj_tiles, (int)list.blocks.size(), set.d_tiles, set.n_tiles, wqd, d_pidx, stride, d_click, d_occ,
+                       n_sm, 0));
+    ck(launch_pack_tiles(model, set.d_tiles, set.n_tiles, wqd, max_tile_sessions, d_pidx, stride, d_click, set.d_tblk, d_status,
+                         true, n_sm, 0));
+    ck(cudaDeviceSynchronize());
+    dfree(d_occ);
+    CK(e);
+    int status = 0;
+    CK(cudaMemcpy(&status, d_status, 4, cudaMemcpyDeviceToHost));
+    if (status) return set_error(MC_ERR_INVALID, "tile packing found a parameter index outside its query's window");
+    return MC_OK;
+}
+
+// The model's own tiles, and the adjoint's, which are their blocks.
+int mc_model::build_tiles() {
+    drop_graph();
+    free_tiles();
+    const std::string misfit = "tile shape does not fit in shared memory (reduce sessions per tile or window)";
+    if (!fused_plan(model, wqd, spt, block, device, false, n, 0, &plan)) return set_error(MC_ERR_INVALID, misfit);
+    auto set = std::make_shared<TileSet>();
+    set->narrow_window = plan.narrow_window;
+    set->narrow_sessions = plan.narrow_sessions;
+    TileList list;
+    cut_tiles(plan.narrow_window, plan.narrow_sessions, list);
     // The adjoint's tiles: every session of a staged block, packed on the first
     // call that takes them (ensure_adjoint_counts).
     std::vector<TileDev>& blocks = list.blocks;
@@ -926,51 +937,61 @@ int mc_model::build_tiles(int layout_model, int narrow_sessions) {
     }
     if (!std::is_sorted(h_adj_begin.begin(), h_adj_begin.end())) h_adj_begin.clear();  // no range lookups
     const int64_t before_adj = bytes;
-    if ((rc = dalloc(&d_adj_tiles, blocks.size(), &bytes))) return rc;
+    if (int rc = dalloc(&d_adj_tiles, blocks.size(), &bytes)) return rc;
     adj_bytes = bytes - before_adj;
-    int* d_occ = nullptr;
-    int64_t scratch = 0;
-    if ((rc = dalloc(&d_occ, blocks.size(), &scratch))) return rc;
-    cudaError_t e = cudaSuccess;
-    auto ck = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-    if (!blocks.empty()) {
-        ck(cudaMemcpyAsync(d_adj_tiles, blocks.data(), blocks.size() * sizeof(TileDev), cudaMemcpyHostToDevice, 0));
-        ck(cudaMemsetAsync(d_occ, 0, blocks.size() * sizeof(int), 0));
-    }
-    ck(launch_tile_occ(model, d_adj_tiles, (int)blocks.size(), d_tiles, n_tiles, wqd, d_pidx, stride, d_click, d_occ, n_sm, 0));
-    ck(launch_pack_tiles(model, d_tiles, n_tiles, wqd, max_tile_sessions, d_pidx, stride, d_click, d_tblk, d_status, true, n_sm, 0));
-    ck(cudaDeviceSynchronize());
-    dfree(d_occ);
-    CK(e);
-    int status = 0;
-    CK(cudaMemcpy(&status, d_status, 4, cudaMemcpyDeviceToHost));
-    if (status) return set_error(MC_ERR_INVALID, "tile packing found a parameter index outside its query's window");
-    tiles_ready = true;
-    tiles_layout = layout_model;
+    if (!blocks.empty()) CK(cudaMemcpy(d_adj_tiles, blocks.data(), blocks.size() * sizeof(TileDev), cudaMemcpyHostToDevice));
+    if (int rc = pack_set(list, *set)) return rc;
+    if (!fused_plan(model, wqd, spt, block, device, false, n, set->widest, &plan)) return set_error(MC_ERR_INVALID, misfit);
+    tiles = std::move(set);
+    bytes += tiles->bytes;
+    return write_fit_desc();
+}
+
+// Tiles for a batch's launches: the model's own where their windows fit the
+// batch's narrow ones and hold as many sessions as the batch as a whole wants
+// per tile; else cut for the batch, which owns them: the model's own launches
+// and other batches keep theirs.  (The model's own at need: a wider window is
+// then one of the batch's wide tiles, and fewer sessions cost speed alone.)
+int mc_model::batch_tiles(const FusedPlan& batch, std::shared_ptr<TileSet>* out) {
+    if (!tiles)
+        if (int rc = build_tiles()) return rc;
+    *out = tiles;
+    if (tiles->narrow_window <= batch.narrow_window && tiles->narrow_sessions >= batch.narrow_sessions) return MC_OK;
+    auto set = std::make_shared<TileSet>();
+    set->narrow_window = batch.narrow_window;
+    set->narrow_sessions = batch.narrow_sessions;
+    TileList list;
+    cut_tiles(batch.narrow_window, batch.narrow_sessions, list);
+    const int rc = pack_set(list, *set);
+    if (rc == MC_ERR_NOMEM) return MC_OK;
+    if (rc) return rc;
+    *out = std::move(set);
     return MC_OK;
 }
 
-FitDev mc_model::make_desc() const {
+FitDev mc_model::make_desc(const TileSet* set) const {
     FitDev f{};
     f.model = model;
     f.mode = mode;
     f.n = n;
     f.stride = stride;
     f.n_qd = n_qd;
-    f.n_chunks = n_echunks;
     f.n_pub = n_pub;
     f.pidx = d_pidx;
     f.click = d_click;
     f.cnt = d_cnt;
     f.cnt16 = d_cnt16;
-    f.tblk = d_tblk;
     f.atr = d_atr;
     f.sat = d_sat;
     f.pub_theta = d_pub_theta;
     f.pub_bins = d_pub_bins;
     f.pub_const = d_pub_const;
-    f.split_bins = d_split_bins;
-    f.split_count = d_split_count;
+    if (set) {
+        f.n_chunks = set->n_echunks;
+        f.tblk = set->d_tblk;
+        f.split_bins = set->d_split_bins;
+        f.split_count = set->d_split_count;
+    }
     f.tiles_done = d_tiles_done;
     f.iter = d_iter;
     f.status = d_status;
@@ -978,7 +999,7 @@ FitDev mc_model::make_desc() const {
 }
 
 int mc_model::write_fit_desc() {
-    FitDev f = make_desc();
+    FitDev f = make_desc(tiles.get());
     CK(cudaMemcpy(d_fit, &f, sizeof(f), cudaMemcpyHostToDevice));
     return MC_OK;
 }
@@ -1361,19 +1382,18 @@ extern "C" int mc_model_configure(mc_model* m, int32_t spt, int32_t wqd, int32_t
     if (m->spt == spt0 && m->wqd == wqd0 && m->block == block0) return MC_OK;
     // Another CTA size alone: the tiles stay if its plan cuts the same ones (16M
     // sessions: 5 ms less per fit that sets its shape after the upload).
-    if (m->uploaded && m->fused_ok && m->tiles_ready && m->spt == spt0 && m->wqd == wqd0) {
+    if (m->uploaded && m->fused_ok && m->tiles && m->spt == spt0 && m->wqd == wqd0) {
         FusedPlan cut, launch;
         if (fused_plan(m->model, m->wqd, m->spt, m->block, m->device, false, m->n, 0, &cut) &&
-            cut.narrow_window == m->plan.narrow_window && cut.narrow_sessions == m->plan.narrow_sessions &&
-            fused_plan(m->model, m->wqd, m->spt, m->block, m->device, false, m->n, m->widest, &launch)) {
+            cut.narrow_window == m->tiles->narrow_window && cut.narrow_sessions == m->tiles->narrow_sessions &&
+            fused_plan(m->model, m->wqd, m->spt, m->block, m->device, false, m->n, m->tiles->widest, &launch)) {
             m->drop_graph();
-            launch.narrow_sessions = cut.narrow_sessions;
             m->plan = launch;
             return MC_OK;
         }
     }
     // Count-path models rebuild tiles only if a batch already made them.
-    if (m->uploaded && m->fused_ok && (!m->d_coff || m->tiles_ready)) return m->build_tiles();
+    if (m->uploaded && m->fused_ok && (!m->d_coff || m->tiles)) return m->build_tiles();
     return MC_OK;
 }
 
@@ -1391,6 +1411,7 @@ static cudaError_t launch_tiles(int model, const FitDev* fits, const TileDev* ti
                                 const SplitDev* splits, WorkState* ws, int wqd, const FusedPlan& plan, int block, int n_sm,
                                 const CountFitDev* cfits, int n_cfits, int count_blocks, cudaStream_t st) {
     const int warps = block / 32;
+    if (plan.cap < fused_narrow_cap(model) * warps) return cudaErrorInvalidValue;  // another kernel's plan
     const int work = std::max(n_wide, (n_tiles - n_wide + warps - 1) / warps) + count_blocks;
     const int grid = std::max(1, std::min(work, plan.ctas * n_sm));
     return launch_em_fused(model, fits, tiles, n_wide, n_tiles, splits, ws, wqd, plan.cap, grid, block, cfits, n_cfits, count_blocks,
@@ -1402,7 +1423,8 @@ static cudaError_t launch_tiles(int model, const FitDev* fits, const TileDev* ti
 static cudaError_t launch_fused_once(mc_model* m, cudaStream_t st) {
     if (m->dense.rows) return launch_em_counts_pbm_dense(m->d_fit, m->dense, m->n_qd, m->n_sm, m->dense_shape, st);
     if (m->d_coff) return launch_em_counts(m->d_fit, m->d_coff, m->d_cent, m->n_qd, m->n_sm, m->count_shape, st);
-    return launch_tiles(m->model, m->d_fit, m->d_tiles, m->n_wide, m->n_tiles, m->d_splits, m->d_ws, m->wqd, m->plan, m->block,
+    const TileSet& t = *m->tiles;
+    return launch_tiles(m->model, m->d_fit, t.d_tiles, t.n_wide, t.n_tiles, t.d_splits, m->d_ws, m->wqd, m->plan, m->block,
                         m->n_sm, nullptr, 0, 0, st);
 }
 
@@ -1855,12 +1877,14 @@ struct mc_batch {
     mc_model::GraphSlot graphs[2];
     cudaStream_t own_stream = nullptr, count_stream = nullptr;
     cudaEvent_t forked = nullptr, joined = nullptr;
+    std::vector<std::shared_ptr<TileSet>> sets;  // the tile fits' packed sessions and split bins
     int64_t bytes = 0;
 
     void release() {
         for (auto& g : graphs) { if (g.exec) cudaGraphExecDestroy(g.exec); g.exec = nullptr; g.iters = -1; }
         settle(d_fits, d_tiles, d_splits, d_ws, d_cfits);
         dfree(d_fits); dfree(d_tiles); dfree(d_splits); dfree(d_ws); dfree(d_cfits);
+        sets.clear();
         if (own_stream) cudaStreamDestroy(own_stream);
         if (count_stream) cudaStreamDestroy(count_stream);
         if (forked) cudaEventDestroy(forked);
@@ -1954,7 +1978,7 @@ extern "C" int mc_batch_create(int n_models, mc_model* const* models, mc_batch**
     for (int i = 0; i < n_models; i++) {
         mc_model* m = models[i];
         // fits[] keeps one entry per model, so a tile's fit index is the model's.
-        fits.push_back(m->make_desc());
+        fits.push_back(m->make_desc(nullptr));
         if (on_counts(m)) {
             CountFitDev c{};
             c.fit = m->d_fit;
@@ -1968,22 +1992,24 @@ extern "C" int mc_batch_create(int n_models, mc_model* const* models, mc_batch**
             cfits.push_back(c);
             continue;
         }
-        if (int rc = m->ensure_tiles(b->plan, b->kernel_model)) { delete b; return rc; }
-        fits.back() = m->make_desc();
-        std::vector<TileDev> t((size_t)m->n_tiles);
-        std::vector<SplitDev> sp((size_t)m->n_splits);
+        std::shared_ptr<TileSet> set;
+        if (int rc = m->batch_tiles(b->plan, &set)) { delete b; return rc; }
+        b->sets.push_back(set);
+        fits.back() = m->make_desc(set.get());
+        std::vector<TileDev> t((size_t)set->n_tiles);
+        std::vector<SplitDev> sp((size_t)set->n_splits);
         cudaError_t e = cudaSuccess;
-        if (!t.empty()) e = cudaMemcpy(t.data(), m->d_tiles, t.size() * sizeof(TileDev), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess && !sp.empty()) e = cudaMemcpy(sp.data(), m->d_splits, sp.size() * sizeof(SplitDev), cudaMemcpyDeviceToHost);
+        if (!t.empty()) e = cudaMemcpy(t.data(), set->d_tiles, t.size() * sizeof(TileDev), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && !sp.empty()) e = cudaMemcpy(sp.data(), set->d_splits, sp.size() * sizeof(SplitDev), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) { delete b; return cuda_fail("batch_create", e); }
         int split_off = (int)splits.size();
-        for (int k = 0; k < m->n_tiles; k++) {
-            TileDev& x = t[(size_t)k];
+        for (TileDev& x : t) {
             x.fit = i;
             if (x.split >= 0) x.split += split_off;
-            (k < m->n_wide ? tiles : narrow).push_back(x);
+            const bool wide = x.qd_count > b->plan.narrow_window;
+            if (wide && x.qd_count <= b->wqd) widest = std::max(widest, x.qd_count);
+            (wide ? tiles : narrow).push_back(x);
         }
-        widest = std::max(widest, m->widest);
         splits.insert(splits.end(), sp.begin(), sp.end());
     }
     if (!plan_for(widest)) return MC_ERR_INVALID;
@@ -2130,7 +2156,7 @@ static AdjointArgs adjoint_args(mc_model* m, int64_t s_begin, int64_t s_count, c
 
 // Sessions grouped by query with tiles built: the adjoint's tile path.
 static bool adjoint_tile_path(const mc_model* m) {
-    return m->fused_ok && m->tiles_ready && !m->h_adj_begin.empty();
+    return m->fused_ok && m->tiles && !m->h_adj_begin.empty();
 }
 
 // The FP32 gradient's per-tile counts (adjoint_counts_kernel) and packed

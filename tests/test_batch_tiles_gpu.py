@@ -81,3 +81,47 @@ def test_em_after_a_refused_shape_is_an_error():
     cm.configure(0, WINDOW, 0)
     cm.em(3)
     _check(cm, api.DBN, sessions, n_qd, 3, "after a refused shape")
+
+
+def _mixed_fits():
+    """DBN and CCM fits with windows between a DBN and a CCM warp's memory, and a
+    DBN fit so large that a batch with it takes more sessions per tile."""
+    small = [(660, 90, 0.8), (410, 60, 0.7), (25, 300, 0.6), (12, 5, 1.0)]
+    large = [(20, 150, 0.9)] * 2000
+    return [(m, *_sessions(q, k)) for k, (m, q) in enumerate([(api.DBN, small), (api.CCM, small), (api.CCM, small[1:]), (api.DBN, large)])]
+
+
+def test_models_alone_after_a_mixed_batch():
+    fits = _mixed_fits()
+    models = [_upload(*f) for f in fits]
+    batch = api.Batch(models)
+    batch.em(2)
+    for f, cm in zip(fits, models):
+        cm.em(2)
+        cm.em_trace(1)
+        _check(cm, *f, 5, "alone after a batch")
+    batch.em(1)
+    for f, cm in zip(fits, models):
+        _check(cm, *f, 6, "batch after alone")
+    batch.close()
+
+
+def test_overlapping_batches_keep_their_tiles():
+    fits = _mixed_fits()
+    models = [_upload(*f) for f in fits]
+    first = api.Batch(models[:2])
+    second = api.Batch(models)
+    third = api.Batch(models[1:])
+    first.em(1)
+    second.em(2)
+    third.em(1)
+    first.em(1)
+    for k, (f, cm) in enumerate(zip(fits, models)):
+        _check(cm, *f, 2 + 2 * (k < 2) + (k > 0), f"overlapping batches, fit {k}")
+    second.close()
+    first.em(1)
+    third.em(1)
+    for k, (f, cm) in enumerate(zip(fits, models)):
+        _check(cm, *f, 2 + 3 * (k < 2) + 2 * (k > 0), f"after one was closed, fit {k}")
+    first.close()
+    third.close()
