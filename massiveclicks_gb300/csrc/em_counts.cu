@@ -385,6 +385,21 @@ __device__ __forceinline__ F2 bytes2(uint32_t w, int i) {
     return add2(pack2(x, y), pack2(-8388608.0f, -8388608.0f));
 }
 
+// The terms of one pair where 1 - a e may be 0 or beyond (0, 1]: a rank without
+// occurrences adds nothing, whatever its reciprocal.  Adds to acc, returns the
+// pair's sum.
+__device__ __noinline__ float dense_pair_any(float a, const float* __restrict__ e, const float* k, F2* acc) {
+    float v0 = 0.0f;
+    for (int r = 0; r < MC_R; r++) {
+        if (k[r] == 0.0f) continue;
+        const float w = k[r] * __fdividef(1.0f, __fmaf_rn(-a, e[r], 1.0f));
+        v0 = __fmaf_rn(w, __fmaf_rn(-a, e[r], a), v0);
+        float* const to = reinterpret_cast<float*>(acc) + r;
+        *to = __fmaf_rn(w, __fmaf_rn(-a, e[r], e[r]), *to);
+    }
+    return v0;
+}
+
 // PBM from dense counts: the unclicked occurrences of a qd at ranks 0..9, so
 // every thread runs the same ten-rank loop and the rank sums stay in registers
 // (no shared atomics); warp sums, then FP64 block sums, then one global atomic
@@ -448,6 +463,14 @@ __global__ void __launch_bounds__(256, 4) em_counts_pbm_dense_kernel(const FitDe
         ee[j] = pack2(e[j].x, e[j].y);
     }
     const F2 one = pack2(1.0f, 1.0f);
+    // Values below `bound` (as bits: 1 while every examination is in [0, 1], as
+    // the M-step leaves them) have 1 - a e in [2^-24, 1] at every rank, and a
+    // rank without occurrences adds 0 times a finite value.  Values that a caller
+    // has set otherwise go to dense_pair_any.
+    uint32_t bound = 0x3F800000u;
+#pragma unroll
+    for (int j = 0; j < MC_R / 2; j++)
+        if (!(e[j].x >= 0.0f && e[j].x <= 1.0f && e[j].y >= 0.0f && e[j].y <= 1.0f)) bound = 0u;
     for (int part = 0;; part++) {
         for (; q < end; q += step) {
             const Row after = row(q + 2 * step);
@@ -464,7 +487,21 @@ __global__ void __launch_bounds__(256, 4) em_counts_pbm_dense_kernel(const FitDe
                 acc[j] = fma2(w, fma2(na, ee[j], ee[j]), acc[j]);
             };
             uint2 n;
-            if (r.w2 != 0xFFFFFFFFu) {
+            const bool wide = r.w2 == 0xFFFFFFFFu;
+            if (__float_as_uint(a) >= bound) {
+                float k[MC_R];
+                n = f.cnt[q];
+#pragma unroll
+                for (int j = 0; j < MC_R; j++)
+                    k[j] = wide ? (float)((__ldg(t.wide + (int64_t)r.w0 * 160 + lane + j / 2 * 32) >> 16 * (j & 1)) & 0xFFFFu)
+                                : (float)(((j < 4 ? r.w0 : j < 8 ? r.w1 : r.w2) >> 8 * (j & 3)) & 0xFFu);
+                F2 sums[MC_R / 2];  // an array whose address is passed on does not stay in registers
+#pragma unroll
+                for (int j = 0; j < MC_R / 2; j++) sums[j] = acc[j];
+                v0 = dense_pair_any(a, reinterpret_cast<const float*>(e), k, sums);
+#pragma unroll
+                for (int j = 0; j < MC_R / 2; j++) acc[j] = sums[j];
+            } else if (!wide) {
                 ranks(0, bytes2(r.w0, 0));
                 ranks(1, bytes2(r.w0, 2));
                 ranks(2, bytes2(r.w1, 0));
