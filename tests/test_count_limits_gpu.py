@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n", [45, 70000])  # counts in bytes, and beyond them
-@pytest.mark.parametrize("batched", [False])
+@pytest.mark.parametrize("batched", [False, True])
 @pytest.mark.parametrize("model", [api.PBM, api.UBM])
 def test_certain_clicks(model, batched, n):
     """Document 0 is attractive for certain; it is clicked at rank 0, whose
