@@ -11,7 +11,7 @@ from oracle import bindings
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [45, 70000])  # counts in bytes, and beyond them
+@pytest.mark.parametrize("n", [45, 2000, 70000])  # PBM counts in bytes, in 16 bits, and beyond the dense table
 @pytest.mark.parametrize("batched", [False, True])
 @pytest.mark.parametrize("model", [api.PBM, api.UBM])
 def test_certain_clicks(model, batched, n):
@@ -25,7 +25,7 @@ def test_certain_clicks(model, batched, n):
     train = api.SessionSet(np.zeros(n, np.int32), docs, docs, clicks)
     cm = api.ClickModel.create(model)
     cm.upload(train, 10)
-    assert cm.fused_path()[0] == ("dense" if model == api.PBM else "counts")
+    assert cm.fused_path()[0] == ("dense" if model == api.PBM and n < 65536 else "counts")
     values = cm.get_parameters()
     values["examination"][:] = np.linspace(0.3, 0.7, len(values["examination"]))
     # rank 0; for UBM its slot, and the first of the table, which no rank has
