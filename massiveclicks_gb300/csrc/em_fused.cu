@@ -415,15 +415,17 @@ __device__ __forceinline__ void reduce_ubm_public(const int (&key)[MC_R], const 
 // click's rank l:
 //   car_r = a_r + gna_r car_{r+1}, car_10 = 0 (compute_exm_car), wanted at the
 //     ranks after l and at l + 1;
-//   Y_j = -g (1 - Pu_j), Pu_j the product of the all-unclicked tail over
-//     documents 0 .. j - 1: Pu_0 = 1, Pu' = Pu - a Eu, Eu_0 = 1, Eu' = Eu gna.
-//     A rank r >= l has the tail R_r = Pu_{9-r}.
+//   Pu_j, the product of the all-unclicked tail over documents 0 .. j - 1:
+//     Pu_0 = 1, Pu' = Pu - a Eu, Eu_0 = 1, Eu' = Eu gna.  A rank r >= l has the
+//     tail R_r = Pu_{9-r}.
 // Both run in one loop: two chains in flight.
 //
 // At a rank after l, with (P, E) the conditional examination (from the last
 // click on) and eps the unconditional one: h = E / (P - g E (1 - R)) gives the
-// public terms g R h = (g + Y) h (numerator) and (1 + Y) h (denominator), summed
-// as h and Y h; the pair's term is a (1 - eps)/(1 - eps car).
+// public terms g R h (numerator) and (1 - g) h + g R h (denominator), summed as h
+// and R h: as h and (1 - R) h, a small R would be lost to cancellation where
+// documents are all attractive (a = 0.999: 2e-4 of the value).  The pair's term is
+// a (1 - eps)/(1 - eps car).
 //
 // The ranks run straight through for all lanes, without a branch on a lane's
 // own l: E is 0 up to its last click, so that h is 0 and P stays 1, takes the
@@ -432,8 +434,8 @@ __device__ __forceinline__ void reduce_ubm_public(const int (&key)[MC_R], const 
 // branches on l kept the ranks' chains from overlapping.)  Three ranks at a
 // time are skipped when no lane has a last click before them.
 struct Ranks {
-    float a[MC_R], gna[MC_R], car[MC_R], Y[MC_R];
-    float P, E, eps, car_l, Y_l;
+    float a[MC_R], gna[MC_R], car[MC_R], Pu[MC_R];
+    float P, E, eps, car_l, R_l;
 };
 
 template <class Ses, class View>
@@ -443,35 +445,35 @@ __device__ __forceinline__ void load_ranks(Ranks& k, const Ses& ses, const View&
         k.a[r] = v.a(ses.at(r));
         k.gna[r] = g * (1.0f - k.a[r]);
     }
-    float c = 0.0f, y = 0.0f, geu = g;
+    float c = 0.0f, pu = 1.0f, eu = 1.0f;
 #pragma unroll
     for (int j = 0; j < MC_R; j++) {
         const int r = MC_R - 1 - j;
-        k.Y[j] = y;
+        k.Pu[j] = pu;
         if (r > 0) {
             c = fmaf(k.gna[r], c, k.a[r]);
             k.car[r] = c;
-            y = fmaf(-k.a[j], geu, y);
-            geu *= k.gna[j];
+            pu = fmaf(-k.a[j], eu, pu);
+            eu *= k.gna[j];
         }
     }
-    k.P = k.eps = 1.0f;
-    k.E = k.car_l = k.Y_l = 0.0f;
+    k.P = k.eps = k.R_l = 1.0f;
+    k.E = k.car_l = 0.0f;
 }
 
 // Rank r >= 1 of a lane with last click l (10: none) and E_l.
 template <class Ses, class View>
-__device__ __forceinline__ void rank_after(Ranks& k, const Ses& ses, const View& v, int r, int l, float E_l, float& sh,
-                                           float& shy) {
-    const float Y = k.Y[MC_R - 1 - r];
+__device__ __forceinline__ void rank_after(Ranks& k, const Ses& ses, const View& v, int r, int l, float g, float E_l, float& sh,
+                                           float& srh) {
+    const float R = k.Pu[MC_R - 1 - r];
     if (l == r - 1) {
         k.E = E_l;
         k.car_l = k.car[r];
-        k.Y_l = k.Y[MC_R - r];
+        k.R_l = k.Pu[MC_R - r];
     }
-    const float h = k.E * rcp(fmaf(k.E, Y, k.P));
+    const float h = k.E * rcp(fmaf(k.E, fmaf(g, R, -g), k.P));
     sh += h;
-    shy = fmaf(h, Y, shy);
+    srh = fmaf(h, R, srh);
     const float x = v.scaled(k.a[r]) * (1.0f - k.eps) * rcp(1.0f - k.eps * k.car[r]);
     if (l < r) v.add_a(ses.at(r), x);
     k.P = fmaf(-k.a[r], k.E, k.P);
@@ -494,7 +496,7 @@ __device__ __forceinline__ int last_click(unsigned m, int& l_min) {
 }
 
 // ---------------------------------------------------------------------------
-// DBN (dbn.cu:207-467); acc: sum of h and of Y h.  Ranks before the last click
+// DBN (dbn.cu:207-467); acc: sum of h and of R h.  Ranks before the last click
 // contribute exactly (1, 1) each and a session without clicks (10, 10) and
 // nothing else: constants of the fit, added at upload (model.cu).
 // ---------------------------------------------------------------------------
@@ -512,7 +514,7 @@ __device__ __forceinline__ void estep_dbn(const Ses& ses, const View& v, float g
 #pragma unroll
             for (int r = 3 * q + 1; r <= 3 * q + 3; r++) {
                 k.eps *= g * (1.0f - k.a[r - 1] * v.s(ses.at(r - 1)));  // g (1 - a) + g a (1 - s)
-                rank_after(k, ses, v, r, l, E_l, acc[0], acc[1]);
+                rank_after(k, ses, v, r, l, g, E_l, acc[0], acc[1]);
             }
         } else {
 #pragma unroll
@@ -521,15 +523,15 @@ __device__ __forceinline__ void estep_dbn(const Ses& ses, const View& v, float g
     }
     // The last click: satisfaction, and gamma with h = (1 - s) / (1 - g (1 - s)(1 - R)).
     if (l < MC_R) {
-        const float h = cs * rcp(fmaf(cs, k.Y_l, 1.0f));
+        const float h = cs * rcp(fmaf(cs, fmaf(g, k.R_l, -g), 1.0f));
         acc[0] += h;
-        acc[1] = fmaf(h, k.Y_l, acc[1]);
+        acc[1] = fmaf(h, k.R_l, acc[1]);
         v.add_s(ol, v.scale * (sl * rcp(1.0f - E_l * k.car_l)));
     }
 }
 
 // ---------------------------------------------------------------------------
-// CCM (ccm.cu:185-478); acc: sum of h and of Y h (tau_1), then the tau_2 and
+// CCM (ccm.cu:185-478); acc: sum of h and of R h (tau_1), then the tau_2 and
 // tau_3 numerators and denominators.
 // ---------------------------------------------------------------------------
 template <class Ses, class View>
@@ -540,18 +542,6 @@ __device__ __forceinline__ void estep_ccm(const Ses& ses, const View& v, float t
     load_ranks(k, ses, v, t1);
     const uint32_t ol = ses.at_lane(l);
     const float al = v.a(ol), ial = 1.0f - al, E_l = __fadd_rn(__fmul_rn(t2, ial), __fmul_rn(t3, al));
-    // The last click's tail R = Pu_{9-l}: 1 + Y_l / t1 would lose a small R to
-    // cancellation.
-    float R = 1.0f;
-    {
-        float pu = 1.0f, eu = 1.0f;
-#pragma unroll
-        for (int j = 0; j < MC_R - 1; j++) {
-            pu = fmaf(-k.a[j], eu, pu);
-            eu *= k.gna[j];
-            if (j + 1 == MC_R - 1 - l) R = pu;
-        }
-    }
     // (1 - a) t1 + a ((1 - a) t2 + a t3), rounded as it always has been: values
     // are compared with those of earlier fits.
     auto step = [&](int r) {
@@ -565,7 +555,7 @@ __device__ __forceinline__ void estep_ccm(const Ses& ses, const View& v, float t
 #pragma unroll
             for (int r = 3 * q + 1; r <= 3 * q + 3; r++) {
                 step(r - 1);
-                rank_after(k, ses, v, r, l, E_l, acc[0], acc[1]);
+                rank_after(k, ses, v, r, l, t1, E_l, acc[0], acc[1]);
             }
         } else {
 #pragma unroll
@@ -585,6 +575,7 @@ __device__ __forceinline__ void estep_ccm(const Ses& ses, const View& v, float t
         acc[2] += p; acc[3] += p;
         acc[4] += q; acc[5] += q;
     }
+    const float R = k.R_l;
     const float k2 = 1.0f - t2 * (1.0f - R), k3 = 1.0f - t3 * (1.0f - R);
     const float B = rcp(ial * k2 + al * k3);
     acc[2] += ial * t2 * R * B;
@@ -601,12 +592,12 @@ __device__ __forceinline__ void estep_ccm(const Ses& ses, const View& v, float t
 __host__ __device__ constexpr int acc_regs(int model) { return model == DBN ? 2 : model == CCM ? 6 : model == UBM ? 0 : MC_R; }
 __device__ __forceinline__ int acc_count(int model) { return model == UBM ? MC_UBM_SLOTS : acc_regs(model); }
 
-// Sums of h and Y h as numerator and denominator terms: g h + Y h and h + Y h.
+// Sums of h and R h as numerator and denominator terms: g R h and (1 - g) h + g R h.
 // v: statistic q of lane q.
 __device__ __forceinline__ double finish_acc(int model, int q, double v, float g) {
     if (model != DBN && model != CCM) return v;
-    const double h = __shfl_sync(FULL_MASK, v, 0), yh = __shfl_sync(FULL_MASK, v, 1);
-    return q == 0 ? fma((double)g, h, yh) : q == 1 ? h + yh : v;
+    const double h = __shfl_sync(FULL_MASK, v, 0), rh = (double)g * __shfl_sync(FULL_MASK, v, 1);
+    return q == 0 ? rh : q == 1 ? fma(1.0 - (double)g, h, rh) : v;
 }
 
 // ---------------------------------------------------------------------------
