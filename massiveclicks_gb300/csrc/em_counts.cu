@@ -385,21 +385,6 @@ __device__ __forceinline__ F2 bytes2(uint32_t w, int i) {
     return add2(pack2(x, y), pack2(-8388608.0f, -8388608.0f));
 }
 
-// The terms of one pair where 1 - a e may be 0 or beyond (0, 1]: a rank without
-// occurrences adds nothing, whatever its reciprocal.  Adds to acc, returns the
-// pair's sum.
-__device__ __noinline__ float dense_pair_any(float a, const float* __restrict__ e, const float* k, F2* acc) {
-    float v0 = 0.0f;
-    for (int r = 0; r < MC_R; r++) {
-        if (k[r] == 0.0f) continue;
-        const float w = k[r] * __fdividef(1.0f, __fmaf_rn(-a, e[r], 1.0f));
-        v0 = __fmaf_rn(w, __fmaf_rn(-a, e[r], a), v0);
-        float* const to = reinterpret_cast<float*>(acc) + r;
-        *to = __fmaf_rn(w, __fmaf_rn(-a, e[r], e[r]), *to);
-    }
-    return v0;
-}
-
 // PBM from dense counts: the unclicked occurrences of a qd at ranks 0..9, so
 // every thread runs the same ten-rank loop and the rank sums stay in registers
 // (no shared atomics); warp sums, then FP64 block sums, then one global atomic
@@ -466,7 +451,7 @@ __global__ void __launch_bounds__(256, 4) em_counts_pbm_dense_kernel(const FitDe
     // Values below `bound` (as bits: 1 while every examination is in [0, 1], as
     // the M-step leaves them) have 1 - a e in [2^-24, 1] at every rank, and a
     // rank without occurrences adds 0 times a finite value.  Values that a caller
-    // has set otherwise go to dense_pair_any.
+    // has set otherwise leave the ranks without occurrences out one by one.
     uint32_t bound = 0x3F800000u;
 #pragma unroll
     for (int j = 0; j < MC_R / 2; j++)
@@ -487,21 +472,7 @@ __global__ void __launch_bounds__(256, 4) em_counts_pbm_dense_kernel(const FitDe
                 acc[j] = fma2(w, fma2(na, ee[j], ee[j]), acc[j]);
             };
             uint2 n;
-            const bool wide = r.w2 == 0xFFFFFFFFu;
-            if (__float_as_uint(a) >= bound) {
-                float k[MC_R];
-                n = f.cnt[q];
-#pragma unroll
-                for (int j = 0; j < MC_R; j++)
-                    k[j] = wide ? (float)((__ldg(t.wide + (int64_t)r.w0 * 160 + lane + j / 2 * 32) >> 16 * (j & 1)) & 0xFFFFu)
-                                : (float)(((j < 4 ? r.w0 : j < 8 ? r.w1 : r.w2) >> 8 * (j & 3)) & 0xFFu);
-                F2 sums[MC_R / 2];  // an array whose address is passed on does not stay in registers
-#pragma unroll
-                for (int j = 0; j < MC_R / 2; j++) sums[j] = acc[j];
-                v0 = dense_pair_any(a, reinterpret_cast<const float*>(e), k, sums);
-#pragma unroll
-                for (int j = 0; j < MC_R / 2; j++) acc[j] = sums[j];
-            } else if (!wide) {
+            if (r.w2 != 0xFFFFFFFFu && __float_as_uint(a) < bound) {
                 ranks(0, bytes2(r.w0, 0));
                 ranks(1, bytes2(r.w0, 2));
                 ranks(2, bytes2(r.w1, 0));
@@ -511,12 +482,32 @@ __global__ void __launch_bounds__(256, 4) em_counts_pbm_dense_kernel(const FitDe
                 n.x = __dp4a(r.w0, 0x01010101u, __dp4a(r.w1, 0x01010101u, __dp4a(r.w2, 0x00000101u, n.y)));
             } else {
                 const uint32_t* p = t.wide + (int64_t)r.w0 * 160 + lane;
-#pragma unroll
-                for (int j = 0; j < MC_R / 2; j++) {
-                    const uint32_t k = __ldg(p + j * 32);
-                    ranks(j, pack2((float)(k & 0xFFFFu), (float)(k >> 16)));
-                }
+                const bool wide = r.w2 == 0xFFFFFFFFu;
                 n = f.cnt[q];
+                if (__float_as_uint(a) < bound) {
+#pragma unroll
+                    for (int j = 0; j < MC_R / 2; j++) {
+                        const uint32_t k = __ldg(p + j * 32);
+                        ranks(j, pack2((float)(k & 0xFFFFu), (float)(k >> 16)));
+                    }
+                } else {
+                    auto term = [&](float k, float x, float& sum) {
+                        if (k == 0.0f) return;
+                        const float w = k * __fdividef(1.0f, __fmaf_rn(-a, x, 1.0f));
+                        v0 = __fmaf_rn(w, __fmaf_rn(-a, x, a), v0);
+                        sum = __fmaf_rn(w, __fmaf_rn(-a, x, x), sum);
+                    };
+#pragma unroll
+                    for (int j = 0; j < MC_R / 2; j++) {
+                        const uint32_t b = (j < 2 ? r.w0 : j < 4 ? r.w1 : r.w2) >> 16 * (j & 1);
+                        const uint32_t k = wide ? __ldg(p + j * 32) : (b & 0xFFu) | (b & 0xFF00u) << 8;
+                        const float2 x = unpack2(ee[j]);
+                        float2 sum = unpack2(acc[j]);
+                        term((float)(k & 0xFFFFu), x.x, sum.x);
+                        term((float)(k >> 16), x.y, sum.y);
+                        acc[j] = pack2(sum.x, sum.y);
+                    }
+                }
             }
             const float v = __fdividef(1.0f + (float)n.y + v0, 2.0f + (float)n.x);
             f.atr[q] = v < MC_TOP ? v : MC_TOP;
