@@ -1338,19 +1338,21 @@ extern "C" int mc_model_upload_test(mc_model* m, int64_t n, const int32_t* pidx,
     CK(cudaSetDevice(m->device));
     m->free_test();
     cudaStream_t st = m->pick(stream);
-    m->n_test = n;
     m->test_stride = std::max<int64_t>(32, (n + 31) / 32 * 32);
     int64_t before = m->bytes, scratch = 0;
     // The rows go to the device as they are, in pieces through one buffer, and
     // become planes there: 4M sessions took 29 ms in a host loop.
     constexpr int64_t kPiece = 1 << 19;
     int32_t* d_rows = nullptr;
-    int rc;
-    if ((rc = dalloc(&m->d_test_pidx, (size_t)(m->test_stride * MC_R), &m->bytes))) return rc;
-    if ((rc = dalloc(&m->d_test_click, (size_t)std::max<int64_t>(n, 1), &m->bytes))) return rc;
-    if ((rc = dalloc(&m->d_eval, MC_R + 1, &m->bytes))) return rc;
+    int rc = dalloc(&m->d_test_pidx, (size_t)(m->test_stride * MC_R), &m->bytes);
+    if (!rc) rc = dalloc(&m->d_test_click, (size_t)std::max<int64_t>(n, 1), &m->bytes);
+    if (!rc) rc = dalloc(&m->d_eval, MC_R + 1, &m->bytes);
     m->test_bytes = m->bytes - before;
-    if ((rc = dalloc(&d_rows, (size_t)std::max<int64_t>(1, std::min(n, kPiece)) * MC_R, &scratch))) return rc;
+    if (!rc) rc = dalloc(&d_rows, (size_t)std::max<int64_t>(1, std::min(n, kPiece)) * MC_R, &scratch);
+    if (rc) {
+        m->free_test();
+        return rc;
+    }
     cudaError_t e = cudaSuccess;
     auto ck = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
     for (int64_t s = 0; s == 0 || s < n; s += kPiece) {
@@ -1361,7 +1363,11 @@ extern "C" int mc_model_upload_test(mc_model* m, int64_t n, const int32_t* pidx,
     if (n) ck(cudaMemcpyAsync(m->d_test_click, click, (size_t)n * 2, cudaMemcpyHostToDevice, st));
     ck(cudaStreamSynchronize(st));
     dfree(d_rows);
-    CK(e);
+    if (e != cudaSuccess) {
+        m->free_test();
+        return cuda_fail("model_upload_test", e);
+    }
+    m->n_test = n;
     return MC_OK;
 }
 
