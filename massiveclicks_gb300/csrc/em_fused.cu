@@ -540,6 +540,18 @@ __device__ __forceinline__ void estep_ccm(const Ses& ses, const View& v, float t
     const int l = last_click(ses.m, l_min);
     Ranks k;
     load_ranks(k, ses, v, t1);
+    // Clicks before the last one: only the tau_2 / tau_3 split depends on the
+    // parameters: u = x / (x + y) and 1 - u = y / (x + y), each from its own
+    // numerator (1 - u formed by subtraction loses the small tau_3 share to
+    // cancellation when tau_3 is near 0).
+    for (unsigned rest = ses.m & ~(1u << l); rest; rest &= rest - 1u) {
+        const float a = v.a(ses.at_lane(31 - __clz(rest & -rest)));
+        const float x = (1.0f - a) * t2, y = a * t3;
+        const float inv = rcp(x + y);
+        const float p = x * inv, q = y * inv;
+        acc[2] += p; acc[3] += p;
+        acc[4] += q; acc[5] += q;
+    }
     const uint32_t ol = ses.at_lane(l);
     const float al = v.a(ol), ial = 1.0f - al, E_l = __fadd_rn(__fmul_rn(t2, ial), __fmul_rn(t3, al));
     // (1 - a) t1 + a ((1 - a) t2 + a t3), rounded as it always has been: values
@@ -563,18 +575,6 @@ __device__ __forceinline__ void estep_ccm(const Ses& ses, const View& v, float t
         }
     }
     if (l == MC_R) return;
-    // Clicks before the last one: only the tau_2 / tau_3 split depends on the
-    // parameters: u = x / (x + y) and 1 - u = y / (x + y), each from its own
-    // numerator (1 - u formed by subtraction loses the small tau_3 share to
-    // cancellation when tau_3 is near 0).
-    for (unsigned rest = ses.m ^ (1u << l); rest; rest &= rest - 1u) {
-        const float a = v.a(ses.at_lane(31 - __clz(rest & -rest)));
-        const float x = (1.0f - a) * t2, y = a * t3;
-        const float inv = rcp(x + y);
-        const float p = x * inv, q = y * inv;
-        acc[2] += p; acc[3] += p;
-        acc[4] += q; acc[5] += q;
-    }
     const float R = k.R_l;
     const float k2 = 1.0f - t2 * (1.0f - R), k3 = 1.0f - t3 * (1.0f - R);
     const float B = rcp(ial * k2 + al * k3);
@@ -1022,6 +1022,12 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
             }
             if (ONE && packed && sc != 0.0f) {
                 const StagedView<true, MODEL, narrow_cap(MODEL)> v{slot, group_cap, sc};
+                estep_chunk<MODEL>(model, ses, v, sl < n_sess, pub, acc, sh.wacc[warp]);
+            } else if (ONE && packed && MODEL == CCM) {
+                // FP32 bins: CCM's as soon as tau_2 or tau_3 is near 1 (out of line,
+                // as below, 1.6M sessions with two clicks each took 78 in place of
+                // 55 us per iteration).
+                const StagedView<false, MODEL, narrow_cap(MODEL)> v{slot, group_cap, 1.0f};
                 estep_chunk<MODEL>(model, ses, v, sl < n_sess, pub, acc, sh.wacc[warp]);
             } else if (packed || direct) {
                 // The other kinds get a copy of the sums: an array whose
