@@ -20,9 +20,9 @@
 //       - owned tile (whole queries): four qd per lane, straight from the bins,
 //         the old values and the click counts, written in place to global
 //         memory (no other tile reads those parameters);
-//       - split tile (part of a large query): one warp folds the bins into the
-//         query's FP64 global bins, and the warp that completes the query's
-//         last tile runs its M-step.
+//       - split tile (part of a large query): the group folds the bins into the
+//         query's FP64 global bins, and the one that completes the query's last
+//         tile runs its M-step.
 // The tiles are cut from blocks of up to 1024 packed sessions and 1536 qd (the
 // shape's), which set the scale of the fixed-point bins: what a pair's bins add
 // up to does not depend on the cut.
@@ -33,7 +33,11 @@
 // 0.203 ms with a warp per tile (CCM: 0.387 and 0.254 ms; 1.6M DBN sessions:
 // 52 and 40 us).  Three tiles in flight per CTA with counted hand-offs instead
 // of the barrier came to 0.236 ms, 0.145 ms of it with the E- and M-steps left
-// out: hand-offs and refills.  Wider windows and direct tiles take a whole CTA.
+// out: hand-offs and refills.  Wider windows, direct tiles, and queries that would
+// be cut at a greater cost (cut_tiles, model.cu) take a whole CTA: up to a block's
+// queries a tile, since a tile costs three barriers (one query each: 20,000
+// queries of 100 sessions and 500 pairs 209 us per iteration, blocks 94, a CTA per
+// block before the warp tiles 100).
 // Bound by instruction issue (about 60% of the slots) and the latencies
 // between; the memory traffic (0.6 GB) is half of its rate.
 //   * public statistics: registers -> every few chunks a warp sum into the
@@ -711,13 +715,12 @@ __device__ __forceinline__ void estep_chunk(int model, const Ses& ses, const Vie
 // Entries of a warp's memory (a narrow tile's arrays).
 __host__ __device__ constexpr int narrow_cap(int model) { return layout_stats(model) > 1 ? 408 : 680; }
 
-// A chunk of a wide tile, or of one that needs FP32 bins, and a chunk of a
-// direct tile: rarer, out of line so that the hot loop stays small in the
-// instruction cache.
-template <int MODEL, bool FX>
-__device__ __noinline__ void estep_chunk_other(int model, const Session ses, unsigned char* slot, int cap, float scale, bool valid,
+// A chunk of a tile that needs FP32 bins, and a chunk of a direct tile: rarer, out
+// of line so that the hot loop stays small in the instruction cache.
+template <int MODEL>
+__device__ __noinline__ void estep_chunk_other(int model, const Session ses, unsigned char* slot, int cap, bool valid,
                                                const float* pub, float* acc, double* wacc) {
-    const StagedView<FX, MODEL, 0> v{slot, cap, scale};
+    const StagedView<false, MODEL, 0> v{slot, cap, 1.0f};
     estep_chunk<MODEL>(model, ses, v, valid, pub, acc, wacc);
 }
 
@@ -776,6 +779,7 @@ struct Shared {
     int index[kWarps][3];                               // of the tiles
     OpenSplit open[kWarps];                             // each warp's last fold, not counted yet
     int warp_fit[kWarps], abort;
+    int last;                                           // a wide split tile was its query's last
     unsigned warp_chunks[kWarps];
 };
 
@@ -785,26 +789,13 @@ __device__ __forceinline__ Shared<MODEL>& cta_shared() {
     return sh;
 }
 
-// A split tile's fold counts once its FP64 adds are done; the warp does that
-// after its next chunk (or before its next fold, or at the end), when the fence
-// no longer waits for them.  The warp that counts the query's last tile runs
-// the query's M-step.
+// M-step of a split query's pairs first, first + step, ..., whose tiles have all
+// been folded; clears its bins.
 template <int MODEL>
-__device__ __noinline__ void count_split(const FitDev* __restrict__ fits) {
-    const int lane = threadIdx.x & 31;
-    const OpenSplit& o = cta_shared<MODEL>().open[threadIdx.x >> 5];
-    __threadfence();
-    __syncwarp();
-    unsigned last = 0;
-    if (lane == 0) last = atomicAdd(o.count, 1u) + 1 == (unsigned)o.split.n_tiles;
-    last = __shfl_sync(FULL_MASK, last, 0);
-    if (!last) return;
-    __threadfence();
-    const SplitDev sp = o.split;
-    const FitDev& f = fits[o.fit];
+__device__ __forceinline__ void mstep_split(const FitDev& f, const SplitDev& sp, int first, int step) {
     const int model = model_of<MODEL>(f), ns = private_stats(model);
     double* const gb = f.split_bins + sp.bin_offset;
-    for (int i = lane; i < sp.qd_count; i += 32) {
+    for (int i = first; i < sp.qd_count; i += step) {
         int64_t q = sp.qd_begin + i;
         uint2 cn = __ldg(f.cnt + q);
         double v0 = ld_cg(gb + (int64_t)i * ns);
@@ -819,8 +810,43 @@ __device__ __noinline__ void count_split(const FitDev* __restrict__ fits) {
         gb[(int64_t)i * ns] = 0.0;
         if (ns > 1) gb[(int64_t)i * ns + 1] = 0.0;
     }
+}
+
+// A narrow split tile's fold counts once its FP64 adds are done; the warp does
+// that after its next chunk (or before its next fold, or at the end), when the
+// fence no longer waits for them.  The warp that counts the query's last tile
+// runs the query's M-step.
+template <int MODEL>
+__device__ __noinline__ void count_split(const FitDev* __restrict__ fits) {
+    const int lane = threadIdx.x & 31;
+    const OpenSplit& o = cta_shared<MODEL>().open[threadIdx.x >> 5];
+    __threadfence();
+    __syncwarp();
+    unsigned last = 0;
+    if (lane == 0) last = atomicAdd(o.count, 1u) + 1 == (unsigned)o.split.n_tiles;
+    last = __shfl_sync(FULL_MASK, last, 0);
+    if (!last) return;
+    __threadfence();
+    mstep_split<MODEL>(fits[o.fit], o.split, lane, 32);
     if (lane == 0) *o.count = 0;
     __syncwarp();
+}
+
+// A CTA counts its fold of a wide split tile (split[0]), and the one that counts
+// the query's last runs its M-step.
+template <int MODEL>
+__device__ __noinline__ void count_wide_split(const FitDev& f) {
+    Shared<MODEL>& sh = cta_shared<MODEL>();
+    const SplitDev& sp = sh.split[0];
+    unsigned* const count = f.split_count + sp.local;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) sh.last = atomicAdd(count, 1u) + 1 == (unsigned)sp.n_tiles;
+    __syncthreads();
+    if (!sh.last) return;
+    __threadfence();
+    mstep_split<MODEL>(f, sp, threadIdx.x, blockDim.x);
+    if (threadIdx.x == 0) *count = 0;
 }
 
 // Adds the sums of a warp (and clears them) to its fit's public bins.
@@ -848,8 +874,9 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
     Shared<MODEL>& sh = cta_shared<MODEL>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_warps = blockDim.x >> 5;
-    const int group = ONE ? warp : 0, gw = ONE ? 0 : warp, group_warps = ONE ? 1 : n_warps;  // gw: this warp in its group
-    const int n_groups = (ONE ? n_warps : 1) * (int)gridDim.x;
+    const int group_warps = ONE ? 1 : n_warps, groups = ONE ? n_warps : 1;
+    const int group = ONE ? warp : 0, gw = ONE ? 0 : warp;  // gw: this warp in its group
+    const int n_groups = groups * (int)gridDim.x;
     const int group_cap = ONE ? narrow_cap(MODEL) : cap;
     const Layout L = make_layout(MODEL, group_cap);
     unsigned char* const slot = smem + (size_t)group * L.bytes;
@@ -858,6 +885,7 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
         if (ONE) __syncwarp();
         else __syncthreads();
     };
+    auto group_all = [&](bool ok) { return ONE ? (bool)__all_sync(FULL_MASK, ok) : (bool)__syncthreads_and(ok); };
     __syncthreads();  // the tiles before, if any, are done with the memory
     for (int i = gw * 32 + lane; i < (int)((L.bytes - L.bins_off) / 16); i += group_warps * 32)
         reinterpret_cast<uint4*>(slot + L.bins_off)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -870,7 +898,7 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
         if (lane < kChunkBytes / 16 - 32) async_copy16(my_chunk + (lane + 32) * 16, src + (lane + 32) * 16);
     };
 
-    // Tile indices (the group's first warp) come in runs of consecutive tiles
+    // Tile indices (the group's last warp) come in runs of consecutive tiles
     // (guided self-scheduling: a run is about 1/4 of the queue left per group,
     // 1 to 8 tiles, estimated from the position this group last took), so a
     // group's tiles are mostly neighbours.  The first run is the group's own by
@@ -881,7 +909,9 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
     auto run_length = [&](int left) { return max(1, min(8, left / (4 * n_groups))); };
     const bool two_rounds = t_end - t_begin <= 2 * n_groups;
     const int first_run = two_rounds ? 1 : run_length(t_end - t_begin);
-    int run_next = t_begin + ((int)blockIdx.x * (ONE ? n_warps : 1) + group) * first_run, run_end = run_next + first_run;
+    // After wide tiles the last CTAs come first: those have had the fewest.
+    const int cta = ONE && t_begin > 0 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+    int run_next = t_begin + (cta * groups + group) * first_run, run_end = run_next + first_run;
     unsigned asked = 0;
     // The next tile's descriptor on its way to tile[slot3].
     auto take_tile = [&](int slot3) {
@@ -905,7 +935,11 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
         }
         if (lane == 0) sh.index[group][slot3] = t;
     };
-    if (gw == 0) {
+    // The group's last warp, which has the fewest chunks, looks ahead (the first
+    // one doing so: 1.6M DBN sessions in queries of 200 over 600 pairs 74 us per
+    // iteration, the last 69; of 42 over 420 pairs 162 and 140).
+    const bool scout = gw == group_warps - 1;
+    if (scout) {
         take_tile(0);
         take_tile(1);
         async_wait_all();
@@ -980,17 +1014,17 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
             if (gw != 0 || lane != 0 || sh.index[group][k3] != g_stall_tile) async_arrive(bar);
         }
         const int next = k3 == 2 ? 0 : k3 + 1;
-        if (gw == 0) take_tile(next == 2 ? 0 : next + 1);
+        if (scout) take_tile(next == 2 ? 0 : next + 1);
         const float sc = fx_scale(tile.max_occ, fx_value_exponent(model, pub));  // 2^shift of the bins, 0: FP32
         // Every lane observes the completed phase itself.
         bool ok = mbar_wait(bar, (uint32_t)k & 1u, status);
-        ok = ONE ? __all_sync(FULL_MASK, ok) : __syncthreads_and(ok);  // the group leaves together
+        ok = group_all(ok);  // the group leaves together
         if (!ok) {
             sh.abort = 1;
             async_wait_all();  // copies still in flight
             break;
         }
-        if (gw == 0) {  // the next tile's values and sessions to L2 (when it is of the same fit)
+        if (scout) {  // the next tile's values and sessions to L2 (when it is of the same fit)
             const TileDev& n = sh.tile[group][next];
             if (n.s_count >= 0 && n.fit == cur_fit && n.qd_count <= window_max) {
                 const unsigned char* const na = reinterpret_cast<const unsigned char*>(f.atr + n.qd_begin);
@@ -1020,14 +1054,14 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
                 __syncwarp();
                 if (c + group_warps < n_chunks) fetch_chunk(chunk + group_warps * kChunkBytes);
             }
-            if (ONE && packed && sc != 0.0f) {
-                const StagedView<true, MODEL, narrow_cap(MODEL)> v{slot, group_cap, sc};
+            if (packed && sc != 0.0f) {
+                const StagedView<true, MODEL, ONE ? narrow_cap(MODEL) : 0> v{slot, group_cap, sc};
                 estep_chunk<MODEL>(model, ses, v, sl < n_sess, pub, acc, sh.wacc[warp]);
-            } else if (ONE && packed && MODEL == CCM) {
+            } else if (packed && MODEL == CCM) {
                 // FP32 bins: CCM's as soon as tau_2 or tau_3 is near 1 (out of line,
                 // as below, 1.6M sessions with two clicks each took 78 in place of
                 // 55 us per iteration).
-                const StagedView<false, MODEL, narrow_cap(MODEL)> v{slot, group_cap, 1.0f};
+                const StagedView<false, MODEL, ONE ? narrow_cap(MODEL) : 0> v{slot, group_cap, 1.0f};
                 estep_chunk<MODEL>(model, ses, v, sl < n_sess, pub, acc, sh.wacc[warp]);
             } else if (packed || direct) {
                 // The other kinds get a copy of the sums: an array whose
@@ -1037,11 +1071,8 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
                 for (int q = 0; q < NA; q++) t[q] = acc[q];
                 if (direct) {
                     estep_chunk_direct<MODEL>(model, f, tile, f.split_bins + sh.split[group].bin_offset, sl, pub, t, sh.wacc[warp]);
-                    __threadfence();  // statistics in global memory, before the split counter is raised
-                } else if (sc != 0.0f) {
-                    estep_chunk_other<MODEL, true>(model, ses, slot, group_cap, sc, sl < n_sess, pub, t, sh.wacc[warp]);
                 } else {
-                    estep_chunk_other<MODEL, false>(model, ses, slot, group_cap, 1.0f, sl < n_sess, pub, t, sh.wacc[warp]);
+                    estep_chunk_other<MODEL>(model, ses, slot, group_cap, sl < n_sess, pub, t, sh.wacc[warp]);
                 }
 #pragma unroll
                 for (int q = 0; q < NA; q++) acc[q] = t[q];
@@ -1052,6 +1083,7 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
                 open = false;
             }
         }
+        if (direct) __threadfence();  // statistics in global memory, before the split counter is raised
         group_sync();  // the bins are complete
 
         const int ns = private_stats(model);
@@ -1095,11 +1127,11 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
                     store(f.sat);
                 }
             }
-        } else if (gw == 0) {
-            if (open) count_split<MODEL>(fits);  // the split tile before
+        } else {
+            if (ONE && open) count_split<MODEL>(fits);  // the split tile before
             double* const gb = f.split_bins + sh.split[group].bin_offset;
             if (!direct) {
-                for (int i = lane; i < tile.qd_count; i += 32)
+                for (int i = gw * 32 + lane; i < tile.qd_count; i += group_warps * 32)
                     for (int q = 0; q < ns; q++) {
                         unsigned char* const p = slot + (i + woff) * 4;
                         unsigned* const bin = reinterpret_cast<unsigned*>(p + (q ? L.bins2_off : L.bins_off));
@@ -1111,8 +1143,12 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
                         if (v != 0.0) atomicAdd(gb + (int64_t)i * ns + q, v);
                     }
             }
-            if (lane == 0) sh.open[warp] = OpenSplit{sh.split[group], f.split_count + sh.split[group].local, tile.fit};
-            open = true;
+            if (ONE) {
+                if (lane == 0) sh.open[warp] = OpenSplit{sh.split[group], f.split_count + sh.split[group].local, tile.fit};
+                open = true;
+            } else {
+                count_wide_split<MODEL>(f);
+            }
         }
     }
     if (open) count_split<MODEL>(fits);

@@ -689,6 +689,23 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
         }
         piece(b, e, tpk);
     };
+    // Whether a query of pk packed sessions is a CTA's.  Cutting it into narrow
+    // tiles costs each a copy of the window, and an FP64 add per bin of it; as one
+    // wide tile per block it costs the CTA's barriers.  Per iteration, narrow
+    // tiles against wide ones, DBN (two bins per pair): queries of 220 to 800
+    // sessions, 200k in all (96 per narrow tile): windows of 30 the same, 50 17.3
+    // and 15.8 us, 100 20.8 and 15.5, 390 38 and 16; 3.2M (512 per tile): 50 63.7
+    // and 71.3, 100 73 and 72, 390 131 and 78.  Of 2200 and 5300 sessions: 200k:
+    // 30 16.4 and 17.3, 70 22 and 18; 3.2M: 150 102 and 107, 300 164 and 140.  CCM
+    // (one bin): about twice these windows.
+    // A query of such a window with two chunks more than narrow_sessions stays a
+    // narrow tile of its own, or a fit of like queries would take a round of each.
+    auto cut_window = [&](int64_t window, bool several_blocks) {
+        return window * ns <= (several_blocks ? std::max(narrow_sessions, 128) : 96 + narrow_sessions / 4);
+    };
+    auto takes_cta = [&](int64_t window, int64_t pk, bool several_blocks) {
+        return window > narrow_window || (pk > narrow_sessions + 64 && !cut_window(window, several_blocks));
+    };
     auto build_range = [&](size_t g0, size_t g1, Part& part) {
         auto tile_of = [&](int split, int64_t b, int64_t e, int64_t lo, int64_t hi, int64_t pk) {
             TileDev t{};
@@ -716,9 +733,8 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
             part.splits.push_back(sp);
             return (int)part.splits.size() - 1;
         };
-        // The tiles of a staged piece of one query (the newest block, or in it).
-        auto query_tiles = [&](int split, int64_t b, int64_t e, int64_t lo, int64_t hi, int64_t pk) {
-            if (hi - lo > narrow_window) return add(part.wide, tile_of(split, b, e, lo, hi, pk));
+        // The narrow tiles of a staged piece of one query (the newest block, or in it).
+        auto narrow_tiles = [&](int split, int64_t b, int64_t e, int64_t lo, int64_t hi, int64_t pk) {
             cut_range(b, e, pk, narrow_sessions,
                       [&](int64_t b1, int64_t e1, int pk1) { add(part.narrow, tile_of(split, b1, e1, lo, hi, pk1)); });
         };
@@ -730,28 +746,38 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
             if (!open) return;
             open = false;
             part.blocks.push_back(cur);
+            // Runs of narrow queries; wide ones with what lies between them.
+            auto is_wide = [&](size_t g) { return takes_cta(seg_hi[g] - seg_lo[g], packed[g - first_seg], false); };
+            size_t last_wide = g_end;  // none
+            for (size_t g = first_seg; g < g_end; g++)
+                if (is_wide(g)) last_wide = g;
             TileDev run{};
-            bool in_run = false;
+            int kind = 0;  // of the open run: 0 none, 1 narrow, 2 wide
             auto end_run = [&]() {
-                if (in_run) add(part.narrow, run);
-                in_run = false;
+                if (kind) add(kind == 2 ? part.wide : part.narrow, run);
+                kind = 0;
             };
             for (size_t g = first_seg; g < g_end; g++) {
                 const int64_t sb = seg_begin[g], se = seg_begin[g + 1], lo = seg_lo[g], hi = seg_hi[g];
                 const int pk = packed[g - first_seg];
-                if (hi - lo > narrow_window || pk > narrow_sessions) {
-                    end_run();
-                    query_tiles(hi - lo > narrow_window ? -1 : new_split(lo, hi, true), sb, se, lo, hi, pk);
-                    continue;
+                if (is_wide(g)) {
+                    if (kind != 2) end_run();
+                } else if (kind != 2) {
+                    if (pk > narrow_sessions && cut_window(hi - lo, false)) {
+                        end_run();
+                        narrow_tiles(new_split(lo, hi, true), sb, se, lo, hi, pk);
+                        continue;
+                    }
+                    if (kind && (run.s_packed + pk > narrow_sessions || hi - run.qd_begin > narrow_window)) end_run();
                 }
-                if (in_run && (run.s_packed + pk > narrow_sessions || hi - run.qd_begin > narrow_window)) end_run();
-                if (!in_run) {
+                if (!kind) {
                     run = tile_of(-1, sb, sb, lo, hi, 0);
-                    in_run = true;
+                    kind = is_wide(g) ? 2 : 1;
                 }
                 run.s_count += (int)(se - sb);
                 run.s_packed += pk;
                 run.qd_count = (int)(hi - run.qd_begin);
+                if (g == last_wide) end_run();
             }
             end_run();
         };
@@ -773,9 +799,11 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
             if (pk > spt || sc > max_sess) {  // staged split query
                 close(g);
                 const int sid = new_split(lo, hi, false);
+                const bool cta = takes_cta(hi - lo, pk, true);  // all of its blocks alike
                 cut_range(sb, sb + sc, pk, spt, [&](int64_t b, int64_t e, int bpk) {
                     part.blocks.push_back(tile_of(sid, b, e, lo, hi, bpk));
-                    query_tiles(sid, b, e, lo, hi, bpk);
+                    if (cta) add(part.wide, part.blocks.back());
+                    else narrow_tiles(sid, b, e, lo, hi, bpk);
                 });
                 continue;
             }
@@ -2009,10 +2037,11 @@ extern "C" int mc_batch_create(int n_models, mc_model* const* models, mc_batch**
         if (e == cudaSuccess && !sp.empty()) e = cudaMemcpy(sp.data(), set->d_splits, sp.size() * sizeof(SplitDev), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) { delete b; return cuda_fail("batch_create", e); }
         int split_off = (int)splits.size();
-        for (TileDev& x : t) {
+        for (int k = 0; k < set->n_tiles; k++) {
+            TileDev& x = t[(size_t)k];
             x.fit = i;
             if (x.split >= 0) x.split += split_off;
-            const bool wide = x.qd_count > b->plan.narrow_window;
+            const bool wide = k < set->n_wide || x.qd_count > b->plan.narrow_window;
             if (wide && x.qd_count <= b->wqd) widest = std::max(widest, x.qd_count);
             (wide ? tiles : narrow).push_back(x);
         }

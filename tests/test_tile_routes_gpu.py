@@ -56,3 +56,34 @@ def _fit_and_check(model, queries, seed, iters, values=None):
 def test_float_bins(queries):
     """Continuations near 1 leave CCM's terms too large for fixed-point bins."""
     _fit_and_check(api.CCM, queries, 1, 2, {"continuation": [0.9, 0.9999, 0.999]})
+
+
+ROUTES = {
+    # both sides of the windows and sessions at which a query is cut (64 sessions per narrow tile in fits this small)
+    "limits": [(w, n) for w in (40, 41, 80, 81) for n in (60, 75, 76, 77, 90, 148, 150, 152, 170, 900)],
+    # runs of wide queries with narrow ones before, between and after them
+    "runs": [(14, 20), (700, 100), (12, 3), (12, 300), (690, 90), (15, 40), (1500, 160), (700, 80), (1200, 150), (11, 2)] * 5,
+    # queries of several blocks, cut or a CTA's, staged and direct
+    "heads": [(30, 3000), (64, 2500), (65, 2500), (300, 2500), (12, 5), (700, 4200), (1600, 2500), (1536, 5000)],
+}
+
+
+@pytest.mark.parametrize("model", [api.CCM, api.DBN])
+@pytest.mark.parametrize("route", ROUTES)
+def test_routes(model, route):
+    _fit_and_check(model, ROUTES[route], len(route), 4)
+
+
+@pytest.mark.parametrize("block", [64, 96, 160, 256])
+def test_blocks_of_other_sizes(block):
+    queries = ROUTES["runs"][:10] + ROUTES["heads"][:3]
+    sessions, n_qd = _sessions(queries, 9)
+    values = []
+    for b in (256, block):
+        cm = api.DBNModel()
+        cm.configure(0, 0, b)
+        cm.upload(sessions, n_qd)
+        cm.em(3)
+        values.append(cm.get_parameters())
+    for name in values[0]:
+        np.testing.assert_allclose(values[1][name], values[0][name], rtol=PARAM_RTOL, atol=PARAM_ATOL, err_msg=name)
