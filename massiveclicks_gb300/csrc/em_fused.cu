@@ -1057,7 +1057,7 @@ __device__ __forceinline__ void run_tiles(const FitDev* __restrict__ fits, const
             if (packed && sc != 0.0f) {
                 const StagedView<true, MODEL, ONE ? narrow_cap(MODEL) : 0> v{slot, group_cap, sc};
                 estep_chunk<MODEL>(model, ses, v, sl < n_sess, pub, acc, sh.wacc[warp]);
-            } else if (packed && MODEL == CCM) {
+            } else if (packed && (MODEL == CCM || MODEL < 0)) {
                 // FP32 bins: CCM's as soon as tau_2 or tau_3 is near 1 (out of line,
                 // as below, 1.6M sessions with two clicks each took 78 in place of
                 // 55 us per iteration).
