@@ -36,7 +36,7 @@
 // out: hand-offs and refills.  Wider windows, direct tiles, and queries that would
 // be cut at a greater cost (cut_tiles, model.cu) take a whole CTA: up to a block's
 // queries a tile, since a tile costs three barriers (one query each: 20,000
-// queries of 100 sessions and 500 pairs 209 us per iteration, blocks 94, a CTA per
+// queries of 100 sessions and 500 pairs 209 us per iteration, runs 103, a CTA per
 // block before the warp tiles 100).
 // Bound by instruction issue (about 60% of the slots) and the latencies
 // between; the memory traffic (0.6 GB) is half of its rate.

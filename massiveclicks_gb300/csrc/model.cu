@@ -629,9 +629,10 @@ static const int kTileSessions = 4096;
 // read directly from global memory in chunks of at most `spt` sessions.  The
 // blocks are the adjoint's tiles, and set the scale of the EM kernel's bins.
 // The EM kernel's tiles are a block's runs of queries of at most narrow_window
-// qd and narrow_sessions packed sessions in all (narrow tiles); a query of more
-// sessions is cut into several, one of a larger window is a wide tile, as is a
-// direct block.  The wide tiles come first (out.n_wide of them), then the
+// qd and narrow_sessions packed sessions in all (narrow tiles).  A query of more
+// sessions is cut into several or, as one of a larger window, taken by a CTA: the
+// block's run of such queries, with those between them, is a wide tile, as is a
+// split query's block or a direct one.  The wide tiles come first (out.n_wide of them), then the
 // narrow ones, each kind in session order; a tile's max_occ holds its block.
 void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) {
     const int ns = private_stats(model);
@@ -691,17 +692,20 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
     };
     // Whether a query of pk packed sessions is a CTA's.  Cutting it into narrow
     // tiles costs each a copy of the window, and an FP64 add per bin of it; as one
-    // wide tile per block it costs the CTA's barriers.  Per iteration, narrow
-    // tiles against wide ones, DBN (two bins per pair): queries of 220 to 800
-    // sessions, 200k in all (96 per narrow tile): windows of 30 the same, 50 17.3
-    // and 15.8 us, 100 20.8 and 15.5, 390 38 and 16; 3.2M (512 per tile): 50 63.7
-    // and 71.3, 100 73 and 72, 390 131 and 78.  Of 2200 and 5300 sessions: 200k:
-    // 30 16.4 and 17.3, 70 22 and 18; 3.2M: 150 102 and 107, 300 164 and 140.  CCM
-    // (one bin): about twice these windows.
-    // A query of such a window with two chunks more than narrow_sessions stays a
-    // narrow tile of its own, or a fit of like queries would take a round of each.
+    // wide tile per block it costs the CTA's barriers, and a fit that has both
+    // kinds of tile a round of each.  Per iteration, narrow tiles against wide
+    // ones, DBN (two bins per pair): queries of 220 to 800 sessions, 200k in all
+    // (96 per narrow tile): windows of 30 the same, 50 17.3 and 15.8 us, 100 20.8
+    // and 15.5, 390 38 and 16; 3.2M (512 per tile): 50 63.7 and 71.3, 100 73 and 72,
+    // 390 131 and 78.  Of 2200 and 5300 sessions: 200k: 30 16.4 and 17.3, 70 22 and
+    // 18; 3.2M: 150 102 and 107, 300 164 and 140.  CCM (one bin): 200k: 100 19.3 and
+    // 19.7, 200 21.6 and 19.6, Zipf fits with windows of 200 26 and 30; 3.2M: 150
+    // 100 and 102, 300 112 and 101; of 2200 and 5300 sessions narrow ones throughout.
+    // A query of a window that is not cut stays a narrow tile of its own up to two
+    // chunks above narrow_sessions, or a fit of like queries would have both kinds.
+    const int wide_from = ns > 1 ? 48 : 192;
     auto cut_window = [&](int64_t window, bool several_blocks) {
-        return window * ns <= (several_blocks ? std::max(narrow_sessions, 128) : 96 + narrow_sessions / 4);
+        return several_blocks ? window * ns * ns <= std::max(2 * narrow_sessions, 256) : window <= wide_from + narrow_sessions / 8;
     };
     auto takes_cta = [&](int64_t window, int64_t pk, bool several_blocks) {
         return window > narrow_window || (pk > narrow_sessions + 64 && !cut_window(window, several_blocks));
