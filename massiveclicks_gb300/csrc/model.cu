@@ -371,7 +371,8 @@ struct FusedPlan {
 
 // False for a shape that is not accepted: its sessions and two windows, with
 // two bin buffers, counts and a byte per entry, have to fit in a CTA's shared
-// memory (a tile needs less; sessions are not staged).  widest: the widest
+// memory.  (A tile needs less; this was the layout of a CTA per tile, and the
+// limit stays so that the same shapes are accepted.)  widest: the widest
 // staged window; one that the memory per CTA at the kernel's occupancy does
 // not hold makes fewer CTAs per SM.
 static bool fused_plan(int model, int wqd, int spt, int block, int device, bool with_counts, int64_t sessions, int widest,
@@ -698,14 +699,15 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
     // (96 per narrow tile): windows of 30 the same, 50 17.3 and 15.8 us, 100 20.8
     // and 15.5, 390 38 and 16; 3.2M (512 per tile): 50 63.7 and 71.3, 100 73 and 72,
     // 390 131 and 78.  Of 2200 and 5300 sessions: 200k: 30 16.4 and 17.3, 70 22 and
-    // 18; 3.2M: 150 102 and 107, 300 164 and 140.  CCM (one bin): 200k: 100 19.3 and
+    // 18; 1.6M: 300 68 and 89; 3.2M: 300 164 and 140.  CCM (one bin): 200k: 100 19.3 and
     // 19.7, 200 21.6 and 19.6, Zipf fits with windows of 200 26 and 30; 3.2M: 150
     // 100 and 102, 300 112 and 101; of 2200 and 5300 sessions narrow ones throughout.
-    // A query of a window that is not cut stays a narrow tile of its own up to two
-    // chunks above narrow_sessions, or a fit of like queries would have both kinds.
+    // Queries of two chunks above narrow_sessions stay narrow tiles of their own, or a
+    // fit of like queries would have both kinds (107 sessions over 200 pairs, CCM:
+    // 22.8 and 16.7); with windows of up to 48 they are cut for the balance.
     const int wide_from = ns > 1 ? 48 : 192;
     auto cut_window = [&](int64_t window, bool several_blocks) {
-        return several_blocks ? window * ns * ns <= std::max(2 * narrow_sessions, 256) : window <= wide_from + narrow_sessions / 8;
+        return several_blocks ? window * ns * ns <= std::max(5 * narrow_sessions / 2, 256) : window <= wide_from + narrow_sessions / 8;
     };
     auto takes_cta = [&](int64_t window, int64_t pk, bool several_blocks) {
         return window > narrow_window || (pk > narrow_sessions + 64 && !cut_window(window, several_blocks));
@@ -767,7 +769,7 @@ void mc_model::cut_tiles(int narrow_window, int narrow_sessions, TileList& out) 
                 if (is_wide(g)) {
                     if (kind != 2) end_run();
                 } else if (kind != 2) {
-                    if (pk > narrow_sessions && cut_window(hi - lo, false)) {
+                    if (pk > narrow_sessions + (hi - lo > 48 ? 64 : 0) && cut_window(hi - lo, false)) {
                         end_run();
                         narrow_tiles(new_split(lo, hi, true), sb, se, lo, hi, pk);
                         continue;
