@@ -384,10 +384,10 @@ def run_ours(args, rank: int, world: int, local: int):
     # counts read; atr, sat written).
     path, n_entries = cm.fused_path()
     if path == "dense":
-        # PBM dense kernel: 20 B of uint16 counts by rank per qd; 8 B occurrence/click
-        # counts, 4 B value read and 4 B value written.
-        design_bytes = 36 * n_qd
-        design_model = "dense count path: 36 B/qd (uint16 counts x10, occurrences/clicks, value read and write)"
+        # PBM dense kernel: 12 B of byte counts by rank and clicks per qd, 4 B value
+        # read and 4 B value written.
+        design_bytes = 20 * n_qd
+        design_model = "dense count path: 20 B/qd (byte counts x10 and clicks, value read and write)"
     elif path == "counts":
         # PBM/UBM count kernel: 4 B per count entry; per qd 4 B offset, 8 B
         # occurrence/click counts, 4 B value read and 4 B value written.

@@ -227,9 +227,10 @@ int mc_model_em_trace(mc_model* m, int32_t n_iterations, double* train_ll, void*
 /* Which kernel one fused iteration of the uploaded model launches: *path = 0
  * the tile kernel over the sessions, 1 the count kernel over the per-(qd, key)
  * occurrence counts built at upload (UBM, and PBM when a count exceeds 16
- * bits), 2 the PBM kernel over dense uint16 [n_qd][10] counts by rank;
- * *n_entries = the number of (qd, key) count entries (0 on the tile path).  The reference has one E-step kernel per
- * model (pbm.cu:191-253, ubm.cu:185-247); this reports which equivalent runs. */
+ * bits), 2 the PBM kernel over dense counts by rank (bytes, 16 bits where they
+ * are larger); *n_entries = the number of (qd, key) count entries (0 on the
+ * tile path).  The reference has one E-step kernel per model (pbm.cu:191-253,
+ * ubm.cu:185-247); this reports which equivalent runs. */
 int mc_model_fused_path(const mc_model* m, int32_t* path, int64_t* n_entries);
 
 /* Testing hook for the timeout path of the fused kernel (the reference stops
@@ -288,7 +289,7 @@ int mc_batch_info(const mc_batch* b, int32_t* n_models, int32_t* n_tiles, int32_
  * the count-path fits (PBM, UBM) after its tiles, one launch per iteration;
  * 0 (the default) runs the count launches beside the tile launches, on a
  * branch of the captured graph.  The default is the faster on 256 mixed fits
- * (0.18 against 0.24 ms per iteration).  Results are the same either way. */
+ * (0.20 against 0.26 ms per iteration).  Results are the same either way. */
 int mc_batch_configure(mc_batch* b, int single_launch);
 
 /* Kernel launches one iteration of the batch makes (0, 1 or 2). */

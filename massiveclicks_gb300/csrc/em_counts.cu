@@ -14,10 +14,12 @@
 // sorting and run-length encoding them gives the entries of each qd (CSR).
 // An iteration is one pass over the qd pairs: a thread takes a qd, evaluates
 // its entries and runs its M-step in place.  The public terms go into
-// per-warp shared bins, then FP64 block sums, then one FP64 global atomic per
-// parameter per block; the block that finishes last runs the public M-step
-// into the other half of the double buffer, as the tile kernel does, so the
-// fit's state (pub_theta, iter) is the same for both paths.
+// per-warp shared bins (dense PBM kernel: registers), then block sums (as
+// integers, count_step.cuh; dense: FP64), then one FP64 global atomic per
+// parameter per block, into one of eight copies of the fit's bins (dense: one);
+// the block that finishes last runs the public M-step into the other half of
+// the double buffer, as the tile kernel does, so the fit's state (pub_theta,
+// iter) is the same for both paths.
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <cub/device/device_radix_sort.cuh>
@@ -296,7 +298,7 @@ cudaError_t build_counts(int model, int64_t n, int64_t stride, int64_t n_qd, con
 // alive entries go into per-warp shared bins.  Bound by the latency of a pair's
 // entries, one after another, and by lane divergence: 64 warps per SM at 32
 // registers hide more of it than prefetches at 40 do (16M UBM sessions: 241 us
-// per iteration, 291 with the next two pairs read ahead), and bins of every
+// per iteration then, 291 with the next two pairs read ahead), and bins of every
 // lane's own in place of atomics leave 28 warps (240 us, with other rounding).
 // A warp per 32 qd with coalesced entry reads, and pairs sorted by their
 // entries, were slower too.

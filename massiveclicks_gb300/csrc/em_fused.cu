@@ -30,8 +30,8 @@
 // then nothing in the loop waits for another warp, and the 24 warps of an SM
 // hide each other's copies and recursions.  Measured per iteration at 16M DBN
 // sessions: 0.351 ms with a CTA of eight warps per tile and a barrier per tile,
-// 0.203 ms with a warp per tile (CCM: 0.387 and 0.254 ms; 1.6M DBN sessions:
-// 52 and 40 us).  Three tiles in flight per CTA with counted hand-offs instead
+// 0.196 ms with a warp per tile (CCM: 0.387 and 0.217 ms; 1.6M DBN sessions:
+// 52 and 41 us).  Three tiles in flight per CTA with counted hand-offs instead
 // of the barrier came to 0.236 ms, 0.145 ms of it with the E- and M-steps left
 // out: hand-offs and refills.  Wider windows, direct tiles, and queries that would
 // be cut at a greater cost (cut_tiles, model.cu) take a whole CTA: up to a block's
@@ -181,8 +181,8 @@ __device__ __forceinline__ float hi16(uint32_t x, float c) { return __int_as_flo
 // A group's shared memory holds one array of `cap` entries per kind of value:
 // float atr, float sat (when satisfaction is a private statistic), uint32
 // cnt16, then one bin array per private statistic.  A window starts at its
-// first qd rounded down to a multiple of four (the bulk copies start on 16
-// bytes, and the M-step takes aligned groups of four): window entry i is entry
+// first qd rounded down to a multiple of four (the copies are of 16 bytes,
+// and the M-step takes aligned groups of four): window entry i is entry
 // i + woff.  The bins are zero between tiles.
 struct Layout {
     uint32_t sat_off, cnt_off, bins_off, bins2_off, bytes;  // of the arrays
@@ -690,8 +690,7 @@ __device__ void flush_public(const FitDev& f, int model, int lane, double v, dou
 template <int MODEL>
 __device__ __forceinline__ int model_of(const FitDev& f) { return MODEL >= 0 ? MODEL : f.model; }
 
-// E-step chunks of a tile (at least one, so that every tile counts), and
-// M-step items of its window: 32 groups of four qd per item.
+// E-step chunks of a tile (at least one, so that every tile counts).
 __device__ __forceinline__ int tile_chunks(int sessions) { return sessions > 32 ? (sessions + 31) >> 5 : 1; }
 
 // One chunk of sessions into the view's bins and the accumulators.
