@@ -1463,9 +1463,9 @@ __global__ void tile_occ_kernel(TileDev* tiles, int n_tiles, const int* __restri
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_tiles; t += gridDim.x * blockDim.x) tiles[t].max_occ = occ[tiles[t].max_occ];
 }
 
-cudaError_t launch_tile_occ(int model, const TileDev* blocks, int n_blocks, TileDev* tiles, int n_tiles, int window_max,
-                            const int32_t* planes, int64_t stride, const uint16_t* click, int* occ, int n_sm, cudaStream_t st) {
-    if (n_tiles == 0) return cudaSuccess;
+cudaError_t launch_block_occ(int model, const TileDev* blocks, int n_blocks, int window_max, const int32_t* planes, int64_t stride,
+                             const uint16_t* click, int* occ, int n_sm, cudaStream_t st) {
+    if (n_blocks == 0) return cudaSuccess;
     const size_t smem = (size_t)window_max * 4;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(block_occ_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1473,6 +1473,11 @@ cudaError_t launch_tile_occ(int model, const TileDev* blocks, int n_blocks, Tile
     }
     block_occ_kernel<<<n_blocks < 8 * n_sm ? n_blocks : 8 * n_sm, 256, smem, st>>>(model, blocks, n_blocks, window_max, planes, stride,
                                                                                   click, occ);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tile_occ(TileDev* tiles, int n_tiles, const int* occ, int n_sm, cudaStream_t st) {
+    if (n_tiles == 0) return cudaSuccess;
     const int g = (n_tiles + 255) / 256;
     tile_occ_kernel<<<g < 8 * n_sm ? g : 8 * n_sm, 256, 0, st>>>(tiles, n_tiles, occ);
     return cudaGetLastError();

@@ -73,12 +73,13 @@ cudaError_t launch_pack_tiles(int model, TileDev* tiles, int n_tiles, int window
                               int64_t stride, const uint16_t* click, unsigned char* tblk, int* status, bool slots,
                               int n_sm, cudaStream_t st);
 
-// Writes the scale of every tile: its max_occ holds the index of its block on
-// entry, and receives the block's largest packed occurrence count of a pair
-// (0 for the blocks of direct tiles, whose occ is not written).  occ: scratch,
-// one per block, zeroed.
-cudaError_t launch_tile_occ(int model, const TileDev* blocks, int n_blocks, TileDev* tiles, int n_tiles, int window_max,
-                            const int32_t* planes, int64_t stride, const uint16_t* click, int* occ, int n_sm, cudaStream_t st);
+// occ[b]: the largest packed occurrence count of a pair of block b (zeroed by the
+// caller; not written for direct blocks).
+cudaError_t launch_block_occ(int model, const TileDev* blocks, int n_blocks, int window_max, const int32_t* planes, int64_t stride,
+                             const uint16_t* click, int* occ, int n_sm, cudaStream_t st);
+// The scale of every tile: its max_occ holds the index of its block on entry, and
+// receives occ of it.
+cudaError_t launch_tile_occ(TileDev* tiles, int n_tiles, const int* occ, int n_sm, cudaStream_t st);
 
 // ---- plain EM (em_plain.cu) -------------------------------------------------
 // The reference's 8-byte device record (data/search.cuh:63-73).
