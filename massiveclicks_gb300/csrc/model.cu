@@ -364,7 +364,8 @@ struct PinnedArray {
 // half of the shape's throughout, 100k sessions took 27 instead of 18 us per
 // iteration: too few warps at work; with half a share, 400k took 29 instead of
 // 21 and 2M 48 instead of 40: tiles cost a copy of the window and a fold.)
-// Wide ones (larger windows, and direct tiles) are a CTA's.
+// Wide ones (larger windows, queries not worth cutting, and direct tiles: see
+// cut_tiles) are a CTA's.
 struct FusedPlan {
     int cap = 8, ctas = 1, narrow_window = 0, narrow_sessions = 1;
 };
